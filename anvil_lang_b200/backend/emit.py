@@ -1052,7 +1052,7 @@ class KernelGen:
         return out
 
     def tc_operands(self, c, touch: bool):
-        """a4 / b4 (four consecutive k of one operand row) and, for the resident template, a_touch / b_touch."""
+        """a4 / b4 (four consecutive k of one operand row) and, for fused attention, a_touch / b_touch."""
         ind = "        "
         dm = self.decode("(uint32_t)m", c.mvars, self.names, ind)
         dn = self.decode("(uint32_t)n", c.nvars, self.names, ind)
@@ -1086,7 +1086,7 @@ class KernelGen:
         M, N, K, NB = c.M, c.N, c.K, c.NB
         nstores = sum(1 for st in k.stmts if isinstance(st, kir.Store))
         variant = tc_variant(c.a_kcontig, M, N, K, nstores)
-        fa4, fb4 = self.tc_operands(c, variant == "pp")
+        fa4, fb4 = self.tc_operands(c, False)
         pp = variant == "pp"
         pair = variant == "pair" or pp
         if pair:                                 # 256 x BN tile per cluster of two CTAs
@@ -1590,7 +1590,7 @@ class HGroupGen:
             kg = KernelGen(gen, k)
             _, _, fe = kg.gemm_functors(c)
             fn = f"{name}_{i}"
-            src += [kg.comment(f"member {i} of a fused launch")] + kg.tc_struct(c, fn, fe, True) + [""]
+            src += [kg.comment(f"member {i} of a fused launch")] + kg.tc_struct(c, fn, fe, False) + [""]
             names.append(fn)
             nlds.append(kg.nld)
         c0 = cs[0]
@@ -1618,10 +1618,8 @@ class HGroupGen:
         first = names[0]
         if kind == "ncat":
             sizes = [c.N for c in cs]
-            f += [f"    __device__ __forceinline__ void a4(int m, int k, int bt, float (&v)[4]) const {{ {first}{{A}}.a4(m, k, bt, v); }}",
-                  f"    __device__ __forceinline__ void a_touch(int m, int k, int bt) const {{ {first}{{A}}.a_touch(m, k, bt); }}"]
+            f += [f"    __device__ __forceinline__ void a4(int m, int k, int bt, float (&v)[4]) const {{ {first}{{A}}.a4(m, k, bt, v); }}"]
             f += dispatch("void b4(int k, int n, int bt, float (&v)[4])", "b4(k, {v}, bt, v)", sizes, "n")
-            f += dispatch("void b_touch(int k, int n, int bt)", "b_touch(k, {v}, bt)", sizes, "n")
             f += dispatch("void epi(int m, int n, int bt, float acc)", "epi(m, {v}, bt, acc)", sizes, "n")
             f += dispatch("void epi_touch(int m, int n, int bt)", "epi_touch(m, {v}, bt)", sizes, "n")
             f += dispatch("void epi_near(int m, int n, int bt)", "epi_near(m, {v}, bt)", sizes, "n")
@@ -1633,8 +1631,6 @@ class HGroupGen:
             sizes = [c.K for c in cs]
             f += dispatch("void a4(int m, int k, int bt, float (&v)[4])", "a4(m, {v}, bt, v)", sizes, "k")
             f += dispatch("void b4(int k, int n, int bt, float (&v)[4])", "b4({v}, n, bt, v)", sizes, "k")
-            f += dispatch("void a_touch(int m, int k, int bt)", "a_touch(m, {v}, bt)", sizes, "k")
-            f += dispatch("void b_touch(int k, int n, int bt)", "b_touch({v}, n, bt)", sizes, "k")
             f += [f"    __device__ __forceinline__ void epi(int m, int n, int bt, float acc) const {{ {first}{{A}}.epi(m, n, bt, acc); }}",
                   f"    __device__ __forceinline__ void epi_touch(int m, int n, int bt) const {{ {first}{{A}}.epi_touch(m, n, bt); }}",
                   f"    __device__ __forceinline__ void epi_near(int m, int n, int bt) const {{ {first}{{A}}.epi_near(m, n, bt); }}",
@@ -1665,9 +1661,7 @@ class HGroupGen:
                 f += [f"    __device__ __forceinline__ int op_seg(int k0, int n0) const {{ return {chain('n0')}; }}",
                       f"    __device__ __forceinline__ int epi_seg(int n0) const {{ return {chain('n0')}; }}"]
                 f += per_member("void a4s(int m, int k, int bt, float (&v)[4])", "a4(m, k, bt, v)", False, "k")
-                f += per_member("void a_touchs(int m, int k, int bt)", "a_touch(m, k, bt)", False, "k")
                 f += per_member("void b4s(int k, int n, int bt, float (&v)[4])", "b4(k, {v}, bt, v)", True, "n")
-                f += per_member("void b_touchs(int k, int n, int bt)", "b_touch(k, {v}, bt)", True, "n")
                 f += per_member("void epi_touchs(int m, int n, int bt)", "epi_touch(m, {v}, bt)", True, "n")
                 f += per_member("void epi_nears(int m, int n, int bt)", "epi_near(m, {v}, bt)", True, "n")
                 f += per_member(f"void epi_loadss(int m, int n, int bt, float (&ld)[{L}])",
@@ -1678,9 +1672,7 @@ class HGroupGen:
                 f += [f"    __device__ __forceinline__ int op_seg(int k0, int n0) const {{ return {chain('k0')}; }}",
                       "    __device__ __forceinline__ int epi_seg(int n0) const { return 0; }"]
                 f += per_member("void a4s(int m, int k, int bt, float (&v)[4])", "a4(m, {v}, bt, v)", True, "k")
-                f += per_member("void a_touchs(int m, int k, int bt)", "a_touch(m, {v}, bt)", True, "k")
                 f += per_member("void b4s(int k, int n, int bt, float (&v)[4])", "b4({v}, n, bt, v)", True, "k")
-                f += per_member("void b_touchs(int k, int n, int bt)", "b_touch({v}, n, bt)", True, "k")
                 f += per_member("void epi_touchs(int m, int n, int bt)", "epi_touch(m, n, bt)", False, "n")
                 f += per_member("void epi_nears(int m, int n, int bt)", "epi_near(m, n, bt)", False, "n")
                 f += per_member(f"void epi_loadss(int m, int n, int bt, float (&ld)[{L}])", "epi_loads(m, n, bt, ld)", False, "n")
