@@ -234,14 +234,17 @@ class Scope:
             return names[lane]
         raise NotImplementedError(k)
 
+    def vec4(self, off: kir.Affine) -> bool:
+        """Are the lanes aligned groups of four consecutive elements at this offset?"""
+        return self.lanes % 4 == 0 and self.lanes >= 4 and an.stride_of(off, self.vv) == 1 and an.aligned4(off, self.vv)
+
     def load(self, e: kir.E, lane) -> str:
         if self.preloaded:
             hit = self.preloaded.get((e.buf.root.id, e.off.key()))
             if hit is not None:
                 return hit
         p = self.kg.ptr(e.buf, False)
-        if self.lanes % 4 == 0 and self.lanes >= 4 and self.depends(e) and an.stride_of(e.off, self.vv) == 1 \
-                and an.aligned4(e.off, self.vv):
+        if self.depends(e) and self.vec4(e.off):
             vkey = ("vec", e.key(), lane // 4)           # lanes come in aligned groups of 4 consecutive elements
             q = self.memo.get(vkey)
             if q is None:
@@ -318,7 +321,7 @@ class Scope:
         k, L = self.kg.k, self.lanes
         p = self.kg.ptr(st.buf, True)
         dt = st.buf.dtype
-        vec_ok = (L % 4 == 0 and L >= 4 and an.stride_of(st.offset, self.vv) == 1 and an.aligned4(st.offset, self.vv))
+        vec_ok = self.vec4(st.offset)
         vals = [self.cast(st.value, dt, lane) for lane in range(L)]
         exclusive = an.exclusive_store(k, st)
         if vec_ok and (not st.accumulate or exclusive):
@@ -1337,6 +1340,9 @@ class RowScope(Scope):
     def key(self, buf, off):
         return (buf.root.id,) + tuple(self.form.canon(off))
 
+    def vec4(self, off: kir.Affine) -> bool:
+        return not self.gg.layout.cyclic and super().vec4(off)
+
     def load(self, e: kir.E, lane) -> str:
         key = self.key(e.buf, e.off)
         hit = self.gg.fwd.get(key)
@@ -1374,12 +1380,12 @@ class RowScope(Scope):
             self.emit(f"if (tt == 0 && live) {p}[{self.affine(st.offset, 0)}] = {vals[0]};")
             return
         self.emit("if (live) {")
-        if an.aligned4(st.offset, self.vv) and L % 4 == 0:
+        if self.vec4(st.offset):
             for g in range(0, L, 4):
-                self.emit(f"    anvil::st4({p} + ({self.affine(st.offset, g)}), make_float4({', '.join(vals[g:g + 4])}));")
+                self.emit(f"    {self.gg.guard(g)}anvil::st4({p} + ({self.affine(st.offset, g)}), make_float4({', '.join(vals[g:g + 4])}));")
         else:
             for lane in range(L):
-                self.emit(f"    {p}[{self.affine(st.offset, lane)}] = {vals[lane]};")
+                self.emit(f"    {self.gg.guard(lane)}{p}[{self.affine(st.offset, lane)}] = {vals[lane]};")
         self.emit("}")
 
 
@@ -1390,6 +1396,7 @@ class RowGroupGen:
         self.gen = gen
         self.forms = forms
         self.dead = dead
+        self.layout = rg.row_layout(forms[0].N)
         self.n = 0
         self.ptrs: dict = {}
         self.fwd: dict = {}              # (root, a, b, const) -> list of C identifiers
@@ -1412,11 +1419,15 @@ class RowGroupGen:
     def rand_varies_with(self, vv) -> bool:
         return False
 
+    def guard(self, slot: int) -> str:
+        """What a store or a reduction of this slot has in front of it where the row does not fill the slots."""
+        return f"if (ok_{slot}) " if self.layout.masked else ""
+
     def generate(self, name: str):
         R, N = self.forms[0].R, self.forms[0].N
-        T = rg.threads_per_row(N)
-        E = N // T
-        RB = rg.THREADS // T
+        lay = self.layout
+        T, E, block = lay.T, lay.E, lay.block
+        RB = block // T
         ind = "    "
         body = []
         for pi, f in enumerate(self.forms):
@@ -1430,8 +1441,8 @@ class RowGroupGen:
                 OP = RED_OP[k.red.op]
                 acc = f"acc{pi}"
                 body.append(f"{ind}float {acc} = {OP}::id<float>();")
-                for v in vals:
-                    body.append(f"{ind}{acc} = {OP}::f({acc}, {v});")
+                for i, v in enumerate(vals):
+                    body.append(f"{ind}{self.guard(i)}{acc} = {OP}::f({acc}, {v});")
                 body.append(f"{ind}{acc} = anvil::row_reduce<{OP}, {T}>({acc}, red_);")
                 tail = RowScope(self, f, 1, ind)
                 tail.acc_name = acc
@@ -1442,8 +1453,8 @@ class RowGroupGen:
                 sc.statements()
                 body += sc.lines
         head = [f"// fused row group: {' + '.join(f.kernel.name for f in self.forms)} | {R} rows x {N} | "
-                f"{T} threads per row, {E} elements each",
-                f"__global__ void __launch_bounds__({rg.THREADS}) {name}(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{"]
+                f"{T} threads per row, {E} elements each{' (masked)' if lay.masked else ''}",
+                f"__global__ void __launch_bounds__({block}) {name}(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{"]
         decls = []
         for rid, (r, w) in sorted(self.ptrs.items()):
             Tn = ctype(r.dtype)
@@ -1452,14 +1463,19 @@ class RowGroupGen:
                 decls.append(f"    {Tn} *b{rid} = ({Tn} *)(A + {off}UL);   // {r.name}{list(r.shape)}")
             else:
                 decls.append(f"    const {Tn} *__restrict__ b{rid} = (const {Tn} *)(A + {off}UL);   // {r.name}{list(r.shape)}")
-        decls += [f"    __shared__ float red_[8];",
+        decls += [f"    __shared__ float red_[16];",
                   f"    const int tt = threadIdx.x % {T};",
                   f"    const long row_ = blockIdx.x * {RB}L + threadIdx.x / {T};",
                   f"    const bool live = row_ < {R}L;",
                   f"    const int row = (int)(live ? row_ : {R - 1}L);"]
         wide = R * N >= (1 << 31)
         for i in range(E):
-            decls.append(f"    const int j_{i} = ({i // 4} * {T} + tt) * 4 + {i % 4};")
+            if not lay.masked:
+                decls.append(f"    const int j_{i} = " + (f"{i * T} + tt;" if lay.cyclic else f"({i // 4} * {T} + tt) * 4 + {i % 4};"))
+            elif lay.cyclic:
+                decls.append(f"    const bool ok_{i} = {i * T} + tt < {N}; const int j_{i} = ok_{i} ? {i * T} + tt : {N - 1};")
+            else:                                        # groups of four lie inside the row or beyond it
+                decls.append(f"    const bool ok_{i} = ({i // 4} * {T} + tt) * 4 < {N}; const int j_{i} = (ok_{i} ? ({i // 4} * {T} + tt) * 4 : {N - 4}) + {i % 4};")
         if any(f.collapsed for f in self.forms):
             ty = "long" if wide else "int"
             for i in range(E):
@@ -1468,7 +1484,7 @@ class RowGroupGen:
         decls.append("    const int j = j_0; (void)j;")
         src = "\n".join(head + decls + body + ["}"])
         blocks = (R + RB - 1) // RB
-        launch = [f"{name}<<<{blocks}, {rg.THREADS}, 0, st>>>(A, sdelta, seed); anvil_rt_count_launches(rt, 1);"]
+        launch = [f"{name}<<<{blocks}, {block}, 0, st>>>(A, sdelta, seed); anvil_rt_count_launches(rt, 1);"]
         return src, launch
 
 

@@ -9,8 +9,8 @@ run of consecutive kernels is fused when every kernel is either
   * a row-wise map:   out[r, j] = f(r, j)         (domain [r, j], or the collapsed form [v] with
                                                    v = r * N + j),
 
-with affine offsets only. T = N / E threads own one row (E = 4 .. 16 elements each, in 128-bit groups
-that are contiguous across threads), keep every row vector they produce in registers, combine their
+with affine offsets only. T threads own one row (up to 16 elements each, in 128-bit groups that are contiguous across
+threads where N is a multiple of 4; the slots beyond N are masked), keep every row vector they produce in registers, combine their
 partial results with a fixed shuffle / shared-memory tree, and go through the kernels in program
 order. A tensor that a later kernel of the group reads at the element this thread wrote is taken
 from the register instead of memory; a tensor that nothing outside the group ever reads is not
@@ -88,11 +88,37 @@ def row_form(k: kir.Kernel, N_hint: int | None = None) -> RowForm | None:
     return None
 
 
-def threads_per_row(N: int) -> int | None:
-    """T threads per row, E = N / T elements each (a multiple of 4, at most 16)."""
+@dataclass
+class RowLayout:
+    """How the T threads of a row hold its N elements: E slots each, slot i of thread t being element (i // 4 * T + t) * 4 + i % 4
+    (`cyclic`: i * T + t). Slots at or beyond N are masked: they read a clamped element and neither reduce nor store."""
+    T: int
+    E: int
+    cyclic: bool
+    masked: bool
+
+    @property
+    def block(self):
+        return max(THREADS, self.T)
+
+
+def row_layout(N: int) -> RowLayout | None:
+    """The smallest T that needs at most 16 slots; None where a row does not fit 512 threads of 16 (or is too short to share).
+
+    Widths that T threads of 4 .. 16 fill exactly (multiples of 128 up to 4096) have no mask. Others were left to one kernel
+    per reduction and map before, each reading the rows again (softmax calls, before -> after: 12504 x 2059 209 -> 64 us, 5391 x
+    441 59 -> 26 us). A width that is no multiple of 4 has unaligned rows: consecutive threads then take consecutive elements, which
+    coalesces 32-bit accesses. 16 slots keep the live row vectors of a softmax or layer-norm gradient in registers at 512
+    threads (128 each); 1024 threads would spill, so rows beyond 8192 stay as they were."""
     for T in (32, 64, 128, 256):
         if N % T == 0 and (N // T) % 4 == 0 and N // T <= 16:
-            return T
+            return RowLayout(T, N // T, False, False)
+    if N < 5:
+        return None
+    for T in (4, 8, 16, 32, 64, 128, 256, 512):
+        E = -(-N // (4 * T)) * 4 if N % 4 == 0 else -(-N // T)
+        if E <= (4 if T < 32 else 16):
+            return RowLayout(T, E, N % 4 != 0, T * E > N)
     return None
 
 
@@ -145,7 +171,7 @@ class Group:
         return True
 
     def worthwhile(self) -> bool:
-        return len(self.forms) >= 2 and any(f.kind == "red" for f in self.forms) and threads_per_row(self.N) is not None
+        return len(self.forms) >= 2 and any(f.kind == "red" for f in self.forms) and row_layout(self.N) is not None
 
 
 def find_groups(kernels: list[kir.Kernel]) -> list[tuple[int, int]]:

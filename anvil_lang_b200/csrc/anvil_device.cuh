@@ -93,13 +93,14 @@ ANVIL_DEV T block_reduce(T v, T *smem) {
     return warp_reduce<Op>(r);
 }
 
-// Reduction over the T threads that share one row (T a power of two, 32 <= T <= 256, rows packed
-// 256 / T to a CTA). Every thread of the row gets the result. Warps are combined in index order.
-// `smem` holds 8 floats. Must be reached by all threads of the CTA.
+// Reduction over the T threads that share one row (T a power of two, 4 <= T <= 512, rows packed
+// into a CTA of at least 256 threads). Every thread of the row gets the result. Warps are combined in index order.
+// `smem` holds 16 floats. Must be reached by all threads of the CTA.
 template <typename Op, int T>
 ANVIL_DEV float row_reduce(float v, float *smem) {
-    v = warp_reduce<Op>(v);
-    if (T == 32) return v;
+#pragma unroll
+    for (int o = (T < 32 ? T : 32) / 2; o > 0; o >>= 1) v = Op::f(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+    if (T <= 32) return v;
     constexpr int WPR = T / 32;                      // warps per row
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
