@@ -910,7 +910,7 @@ class KernelGen:
         fn = f"G{k.id}"
         if tc_eligible(c):
             return self.gen_gemm_tc(base, c, fn, fa, fb, fe, S)
-        return self.gen_gemm_simt(base, c, fn, fa, fb, fe, S, tiles, AK, BNC)
+        return self.gen_gemm_simt(base, c, fn, fa, fb, fe, S, AK, BNC)
 
     def gemm_functors(self, c):
         """The functor methods every contraction template takes: a / b (one operand element), epi (the statements on
@@ -996,22 +996,24 @@ class KernelGen:
         self.nld = nld
         return fa, fb, fe
 
-    def gen_gemm_simt(self, base, c, fn, fa, fb, fe, S, tiles, AK, BNC):
+    def gen_gemm_simt(self, base, c, fn, fa, fb, fe, S, AK, BNC):
         k = self.k
         M, N, K, NB = c.M, c.N, c.K, c.NB
-        src = [self.comment(f"contraction M={M} N={N} K={K} batch={NB} (CUDA-core tiles, split {S})"),
+        TM, TN = simt_tile(M, N, NB * S)
+        tiles = -(-M // TM) * -(-N // TN)
+        src = [self.comment(f"contraction M={M} N={N} K={K} batch={NB} ({TM} x {TN} CUDA-core tiles, split {S})"),
                f"struct {fn} {{", "    char *__restrict__ A;",
                f"    static constexpr int M = {M}, N = {N}, K = {K}, NB = {NB};",
                f"    static constexpr float ALPHA = {flit(c.alpha)};"] + fa + fb + fe + ["};"]
         launch = []
         if S == 1:
-            src += [f"__global__ void __launch_bounds__(256) {base}(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{",
-                    f"    anvil::gemm_simt_tile<{fn}, {AK}, {BNC}, 1>({fn}{{A}}, nullptr);", "}"]
+            src += [f"__global__ void __launch_bounds__(256, 2) {base}(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{",
+                    f"    anvil::gemm_simt_tile<{fn}, {AK}, {BNC}, 1, {TM}, {TN}>({fn}{{A}}, nullptr);", "}"]
             launch.append(self.launch_line(base, f"dim3({tiles}, {NB})", 256))
         else:
             soff = self.scratch(4 * M * N * NB * S)
-            src += [f"__global__ void __launch_bounds__(256) {base}_part(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{",
-                    f"    anvil::gemm_simt_tile<{fn}, {AK}, {BNC}, {S}>({fn}{{A}}, (float *)(A + {soff}UL));", "}",
+            src += [f"__global__ void __launch_bounds__(256, 2) {base}_part(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{",
+                    f"    anvil::gemm_simt_tile<{fn}, {AK}, {BNC}, {S}, {TM}, {TN}>({fn}{{A}}, (float *)(A + {soff}UL));", "}",
                     f"__global__ void __launch_bounds__(256) {base}(char *__restrict__ A, uint32_t sdelta, uint32_t seed_) {{",
                     f"    anvil::gemm_split_finish<{fn}, {S}>({fn}{{A}}, (const float *)(A + {soff}UL));", "}"]
             launch.append(self.launch_line(base + "_part", f"dim3({tiles}, {NB * S})", 256))
@@ -1165,6 +1167,17 @@ class KernelGen:
         self.notes = f"gemm tc {NB}x{M}x{N}x{K} S{S}" + (" A-tmem" if ts else " pp" if pp else " pair" if pair else "")
         self.contraction = c
         return "\n".join(src), launch
+
+
+def simt_tile(M: int, N: int, parts: int) -> tuple[int, int]:
+    """Tile of the CUDA-core template: the widest that the output's columns do not leave mostly empty and that gives every SM
+    a CTA, else 32 x 32 (the sums are the same for every tile). With 128 x 128 for all, 512 x 128 x 128 ran on four CTAs:
+    the small transformer's step, three dozen such products, took 1085 us and takes 577; the convolution gradient 21632 x 32 x
+    576 wasted three quarters of its tile (CNN step 314 -> 290 us)."""
+    for tm, tn in ((128, 32), ) if N <= 32 else ((64, 64), ) if N <= 64 else ((128, 128), (64, 64)):
+        if -(-M // tm) * -(-N // tn) * parts >= 148:
+            return tm, tn
+    return 32, 32
 
 
 def os_environ(name: str, default: str) -> str:

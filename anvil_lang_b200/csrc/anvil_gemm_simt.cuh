@@ -2,9 +2,9 @@
 //
 // The reference runs a contraction as one thread per output element with a serial loop over k that
 // re-reads A and B from global memory (anvil/backend/cuda.py:282-313). This template is the
-// general-purpose replacement: 128 x 128 x 16 tiles staged in shared memory, an 8 x 8 register tile
-// per thread read with 128-bit shared loads, double-buffered global -> register -> shared
-// prefetch. It takes a generated functor F, so operand prologues (max(x, 0), constant scales,
+// general-purpose replacement: tiles of 128, 64 or 32 rows and columns staged in shared memory, a register tile of 1/16 of
+// each side per thread read with vector shared loads, double-buffered global -> register -> shared
+// prefetch, two columns per packed FMA. It takes a generated functor F, so operand prologues (max(x, 0), constant scales,
 // gathered rows) and fused epilogues (bias, activation, residual, optimizer update, several stores)
 // need no extra passes:
 //
@@ -19,61 +19,82 @@
 
 namespace anvil {
 
-constexpr int GS_BM = 128, GS_BN = 128, GS_BK = 16, GS_THREADS = 256, GS_PAD = 4;
+constexpr int GS_THREADS = 256;
+constexpr int GS_KSTEP = 16;               // split ranges are multiples of this, whatever the tile
+
+template <int V> __device__ __forceinline__ void gs_read(const float *p, float (&v)[V]) {
+    if constexpr (V == 2) { const float2 x = *reinterpret_cast<const float2 *>(p); v[0] = x.x; v[1] = x.y; }
+    else { const float4 x = *reinterpret_cast<const float4 *>(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+}
 
 // AK: A is contiguous along k (else along m). BNC: B is contiguous along n (else along k).
 // SPLIT > 1: blockIdx.z / NB selects a k range and the tile goes to `partial` instead of f.epi.
-template <class F, bool AK, bool BNC, int SPLIT>
+// TM x TN: the tile. Every tile adds the same products in the same order, so the results do not depend on it. A product
+// with few 128-wide tiles leaves most of the chip idle and pays a global load's latency per 16 k (512 x 128 x 128: four
+// CTAs, eight round trips); 32-wide tiles spread it over 16 times the CTAs with 64 k per round trip. A narrow output
+// (convolution channels) would multiply zeros in three quarters of a 128-wide tile. Large products keep 128 x 128: 64 FMAs
+// per 4 shared loads against 16 per 2 and 4 per 2.
+template <class F, bool AK, bool BNC, int SPLIT, int TM = 128, int TN = 128>
 __device__ __forceinline__ void gemm_simt_tile(const F &f, float *__restrict__ partial) {
-    __shared__ __align__(16) float As[2][GS_BK][GS_BM + GS_PAD];
-    __shared__ __align__(16) float Bs[2][GS_BK][GS_BN + GS_PAD];
+    constexpr int KB = 2048 / (TM > TN ? TM : TN), PA = TM * KB / GS_THREADS, PB = TN * KB / GS_THREADS;
+    constexpr int RM = TM / 16, VM = RM < 4 ? RM : 4, GM = RM / VM;  // rows per thread: GM groups of VM, 64 apart
+    constexpr int RN = TN / 16, VN = RN < 4 ? RN : 4, GN = RN / VN;  // columns likewise
+    __shared__ __align__(16) float As[2][KB][TM + (TM == 32 ? 2 : 4)];
+    __shared__ __align__(16) float Bs[2][KB][TN + (TN == 32 ? 2 : 4)];
     constexpr int M = F::M, N = F::N, K = F::K;
-    constexpr int TILES_N = (N + GS_BN - 1) / GS_BN;
+    constexpr int TILES_N = (N + TN - 1) / TN;
     const int t = threadIdx.x;
     const int tile_m = blockIdx.x / TILES_N, tile_n = blockIdx.x % TILES_N;
     const int bt = SPLIT > 1 ? blockIdx.y / SPLIT : blockIdx.y;
     const int sp = SPLIT > 1 ? blockIdx.y % SPLIT : 0;
-    constexpr int KCH = ((K + SPLIT - 1) / SPLIT + GS_BK - 1) / GS_BK * GS_BK;   // k range of one split
+    constexpr int KCH = ((K + SPLIT - 1) / SPLIT + GS_KSTEP - 1) / GS_KSTEP * GS_KSTEP;   // k range of one split
     const int k_begin = sp * KCH;
     const int k_end = min(K, k_begin + KCH);
-    const int m0 = tile_m * GS_BM, n0 = tile_n * GS_BN;
+    const int m0 = tile_m * TM, n0 = tile_n * TN;
 
-    float ra[8], rb[8];                    // global -> register staging (8 elements per operand per thread)
+    float ra[PA], rb[PB];                  // global -> register staging
+    // element r of this thread: consecutive threads along k where the operand is contiguous along k, else along its rows
+    auto at = [&](bool along_k, int rows, int r, int &row, int &k) {
+        if (along_k) { k = t % KB; row = t / KB + (GS_THREADS / KB) * r; }
+        else { row = t % rows; k = t / rows + (GS_THREADS / rows) * r; }
+    };
     auto fetch = [&](int k0) {
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
+        for (int r = 0; r < PA; r++) {
             int mm, kk;
-            if (AK) { kk = t % GS_BK; mm = t / GS_BK + (GS_THREADS / GS_BK) * r; }
-            else { mm = t % GS_BM; kk = t / GS_BM + (GS_THREADS / GS_BM) * r; }
+            at(AK, TM, r, mm, kk);
             const int m = m0 + mm, k = k0 + kk;
             ra[r] = (m < M && k < k_end) ? f.a(m, k, bt) : 0.0f;
-            int nn, kb;
-            if (BNC) { nn = t % GS_BN; kb = t / GS_BN + (GS_THREADS / GS_BN) * r; }
-            else { kb = t % GS_BK; nn = t / GS_BK + (GS_THREADS / GS_BK) * r; }
-            const int n = n0 + nn, k2 = k0 + kb;
-            rb[r] = (n < N && k2 < k_end) ? f.b(k2, n, bt) : 0.0f;
+        }
+#pragma unroll
+        for (int r = 0; r < PB; r++) {
+            int nn, kk;
+            at(!BNC, TN, r, nn, kk);
+            const int n = n0 + nn, k = k0 + kk;
+            rb[r] = (n < N && k < k_end) ? f.b(k, n, bt) : 0.0f;
         }
     };
     auto stage = [&](int buf) {
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
+        for (int r = 0; r < PA; r++) {
             int mm, kk;
-            if (AK) { kk = t % GS_BK; mm = t / GS_BK + (GS_THREADS / GS_BK) * r; }
-            else { mm = t % GS_BM; kk = t / GS_BM + (GS_THREADS / GS_BM) * r; }
+            at(AK, TM, r, mm, kk);
             As[buf][kk][mm] = ra[r];
-            int nn, kb;
-            if (BNC) { nn = t % GS_BN; kb = t / GS_BN + (GS_THREADS / GS_BN) * r; }
-            else { kb = t % GS_BK; nn = t / GS_BK + (GS_THREADS / GS_BK) * r; }
-            Bs[buf][kb][nn] = rb[r];
+        }
+#pragma unroll
+        for (int r = 0; r < PB; r++) {
+            int nn, kk;
+            at(!BNC, TN, r, nn, kk);
+            Bs[buf][kk][nn] = rb[r];
         }
     };
 
     const int tx = t % 16, ty = t / 16;
-    float acc[8][8];
+    float2 acc[RM][RN / 2];                // two neighbouring columns per packed FMA
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < RM; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < RN / 2; j++) acc[i][j] = make_float2(0.0f, 0.0f);
 
     int buf = 0;
     if (k_begin < k_end) {
@@ -81,21 +102,23 @@ __device__ __forceinline__ void gemm_simt_tile(const F &f, float *__restrict__ p
         stage(0);
     }
     __syncthreads();
-    for (int k0 = k_begin; k0 < k_end; k0 += GS_BK) {
-        const bool more = k0 + GS_BK < k_end;
-        if (more) fetch(k0 + GS_BK);
+    for (int k0 = k_begin; k0 < k_end; k0 += KB) {
+        const bool more = k0 + KB < k_end;
+        if (more) fetch(k0 + KB);
+#pragma unroll 16
+        for (int kk = 0; kk < KB; kk++) {
+            float av[GM][VM], bv[GN][VN];
 #pragma unroll
-        for (int kk = 0; kk < GS_BK; kk++) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4 + 64]);
-            const float4 b0 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4 + 64]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            for (int g = 0; g < GM; g++) gs_read<VM>(&As[buf][kk][ty * VM + 64 * g], av[g]);
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+            for (int g = 0; g < GN; g++) gs_read<VN>(&Bs[buf][kk][tx * VN + 64 * g], bv[g]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
+            for (int i = 0; i < RM; i++)
+#pragma unroll
+                for (int j = 0; j < RN; j += 2) {
+                    const float a = av[i / VM][i % VM];
+                    acc[i][j / 2] = __ffma2_rn(make_float2(a, a), make_float2(bv[j / VN][j % VN], bv[j / VN][j % VN + 1]), acc[i][j / 2]);
+                }
         }
         if (more) stage(buf ^ 1);
         __syncthreads();
@@ -103,15 +126,16 @@ __device__ __forceinline__ void gemm_simt_tile(const F &f, float *__restrict__ p
     }
 
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int m = m0 + ty * 4 + (i & 3) + (i >> 2) * 64;
+    for (int i = 0; i < RM; i++) {
+        const int m = m0 + ty * VM + i % VM + (i / VM) * 64;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int n = n0 + tx * 4 + (j & 3) + (j >> 2) * 64;
+        for (int j = 0; j < RN; j++) {
+            const int n = n0 + tx * VN + j % VN + (j / VN) * 64;
             if (n >= N) continue;
-            if (SPLIT > 1) partial[(((long)bt * SPLIT + sp) * M + m) * N + n] = acc[i][j];
-            else f.epi(m, n, bt, acc[i][j] * F::ALPHA);
+            const float v = j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x;
+            if (SPLIT > 1) partial[(((long)bt * SPLIT + sp) * M + m) * N + n] = v;
+            else f.epi(m, n, bt, v * F::ALPHA);
         }
     }
 }
