@@ -496,8 +496,10 @@ class KernelGen:
         blocks = (ON + OX - 1) // OX
         S = 1
         per_thread = RN // (RY * L)
-        if blocks < 148 and per_thread >= 64:
-            S = max(1, min(296 // blocks, per_thread // 32, 64))
+        if blocks < 592 and per_thread >= 64:
+            # a thread keeps four loads in flight: eight CTAs per SM cover their latency, two did not (CNN step, whose bias and
+            # first-layer gradients reduce 86528 positions to 32 and 288 values: 290 -> 277 us; MLP Adam step 177 -> 170)
+            S = max(1, min(1184 // blocks, per_thread // 16, 64))
         return ("coop", layout, OX, RY, L, S)
 
     def vec_width_domain(self) -> int:
@@ -1274,7 +1276,7 @@ def use_tma() -> bool:
     B200 it is slower than the converters' own loads (16384 x 512 x 512: 72 us against 49 us). The stage ring holds three
     66 KB stages (hi and lo tiles of both operands, 198 of 227 KB), so only one block's copy can be in flight while the
     tensor core works on one stage and the converters make lo for the next, and a copy takes longer than a block's MMAs;
-    the load path keeps two blocks' operands in registers and asks L2 for four more. ANVIL_B200_TMA=1 turns it on."""
+    the load path keeps two blocks' operands in registers. ANVIL_B200_TMA=1 turns it on."""
     import os
     return os.environ.get("ANVIL_B200_TMA", "0") == "1"
 

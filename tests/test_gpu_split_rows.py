@@ -1,0 +1,41 @@
+"""Row reductions on both sides of the rule that splits them over CTAs, against float64."""
+import numpy as np
+import pytest
+
+from anvil_lang_b200 import kir
+from anvil_lang_b200.backend import emit
+from kirbuild import E, F32, Affine, Kernel, KernelStmt, Reduction, Store, buf, load, nid, var
+
+CASES = [        # rows, row length, split (64 elements per thread of 256 from 16384 on; fewer than 592 rows)
+    (591, 16387, 2), (592, 16387, 1), (300, 16383, 1), (288, 16387, 4), (148, 16385, 4), (3, 65537, 16), (1, 300001, 64),
+]
+
+
+def program(R, N):
+    x, y = buf("x", (R, N), kind="input"), buf("y", (R,), kind="output")
+    r, j = var("r", R), var("j", N)
+    k = Kernel(nid(), f"k{nid()}", "row sum", [r], [Store(y, Affine(0, [(r, 1)]), E("acc", F32), False)],
+               Reduction([j], "sum", load(x, [(r, N), (j, 1)])))
+    return kir.Program(kir.Block([KernelStmt(k)]), [x, y], "row sum"), x, y
+
+
+@pytest.mark.parametrize("R,N,S", CASES)
+def test_split(R, N, S):
+    note = emit.generate(program(R, N)[0], 0)[1].kernel_notes[0]
+    assert note == (f"split row 1x256 L1 S{S}" if S > 1 else "coop row 1x256 L1")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,N,S", CASES)
+def test_row_sums(R, N, S):
+    """A thread adds at most N / (256 S) values in a row, then eight tree levels and S parts: the error of a sum of positive
+    values stays below (N / (256 S) + 8 + S) roundings of 2^-24."""
+    from anvil_lang_b200.program import DeviceProgram
+    prog, x, y = program(R, N)
+    dp = DeviceProgram(prog, seed=0, graphs=False)
+    a = np.random.default_rng(N).random((R, N), dtype=np.float32)
+    dp.write(x, a)
+    assert dp.run()[0] == 0
+    got, want = dp.read(y).astype(np.float64), a.astype(np.float64).sum(axis=1)
+    dp.close()
+    assert (np.abs(got - want) <= (N / (256 * S) + 8 + S) * 2.0 ** -24 * want).all()
