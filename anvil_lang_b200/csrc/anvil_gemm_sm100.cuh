@@ -897,7 +897,7 @@ __device__ __forceinline__ void gemm_tc_pair_tile(const F &f, float *__restrict_
 // What bounds it: the converters (the same kernel with one MMA per block takes 222 of 243 us at 8192 x 4096 x 1024; with
 // no global loads 228). Measured alone, chains of 512 and more mixed (below), before -> after these two and the mixed split:
 // 8192 x 4096 x 1024 288 -> 243 us, 16384 x 2048 x 512 148 -> 127, 16384 x 512 x 2048 155 -> 141, 512 x 2048 x 16384
-// 160 -> 142. Asking L2 for operands some blocks ahead cost more issue slots than it hid once the loads had a block's
+// 160 -> 142 (129 with bare loads, below). Asking L2 for operands some blocks ahead cost more issue slots than it hid once the loads had a block's
 // time (252, 131, 156, 140 us with it).
 // ACCS = 2 keeps the correction accumulator (one TMEM buffer of 512 columns: the next tile's MMAs wait
 // for the epilogue's loads, the converters do not). ACCS = 1 adds all products into one accumulator,
@@ -1084,6 +1084,13 @@ __device__ __forceinline__ void gemm_tc_pair_persistent(const F &f, float *__res
     constexpr int KCH = ((K + SPLIT - 1) / SPLIT + BK - 1) / BK * BK;
     constexpr int NST = STAGES, G = PP_CONV_GROUPS;
     constexpr bool MIXED = pp_mixed(KCH);
+    // Both operands read along their rows (a weight gradient): four scalar loads per chunk, and the guards in front of them
+    // cost as much as they do. There a side that the tiles fill exactly has none, and a turn without a next block skips the
+    // fetch: 512 x 2048 x 16384 140 -> 129 us. With an operand read along k the same made the kernel slower (16384 x 2048 x
+    // 512 122 -> 131 us, 16384 x 512 x 2048 141 -> 152): predicated vector loads stay where they are written, bare ones move.
+    constexpr bool ROWS = !AK && !BKC;
+    constexpr bool FULL_M = ROWS && M % (2 * BM) == 0, FULL_N = ROWS && N % BN == 0;
+    constexpr bool FULL_K = ROWS && K % BK == 0 && (SPLIT - 1) * KCH < K;        // (a k range may start beyond K where splits round up)
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const uint32_t rank = cluster_ctarank();
     const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
@@ -1205,14 +1212,14 @@ __device__ __forceinline__ void gemm_tc_pair_persistent(const F &f, float *__res
             int row, kc;
             TileMapPP<AK, BM>::at(tc, p, row, kc);
             const int m = it.m0 + row, k = k0 + kc * 4;
-            if (m < M && k < k_end) f_a4<decltype(S_)::value>(f, m, k, it.bt, va[p]);
+            if ((FULL_M || m < M) && (FULL_K || k < k_end)) f_a4<decltype(S_)::value>(f, m, k, it.bt, va[p]);
             else { va[p][0] = va[p][1] = va[p][2] = va[p][3] = 0.0f; }
         };
         auto fetch_b = [&](auto S_, const Item &it, int k0, int k_end, int p) {
             int row, kc;
             TileMapPP<BKC, BH>::at(tc, p, row, kc);
             const int n = it.nb0 + row, k = k0 + kc * 4;
-            if (n < N && k < k_end) f_b4<decltype(S_)::value>(f, k, n, it.bt, vb[p]);
+            if ((FULL_N || n < N) && (FULL_K || k < k_end)) f_b4<decltype(S_)::value>(f, k, n, it.bt, vb[p]);
             else { vb[p][0] = vb[p][1] = vb[p][2] = vb[p][3] = 0.0f; }
         };
         // The TMA copies of block (it, kb) into stage s: eight 16-byte columns per operand; rows or k beyond the matrix read as zeros
@@ -1261,7 +1268,8 @@ __device__ __forceinline__ void gemm_tc_pair_persistent(const F &f, float *__res
                     for (int p = 0; p < BM / 32; p += PutA::STEP) {
                         PutA::put(st, tc, p, va);
 #pragma unroll
-                        for (int i = 0; i < PutA::STEP; i++) fetch_a(S_, it, k0, k_end, p + i);
+                        for (int i = 0; i < PutA::STEP; i++)
+                            if (!ROWS || w < WORK) fetch_a(S_, it, k0, k_end, p + i);
                     }
                 }
                 if (!TMA_B) {
@@ -1269,7 +1277,8 @@ __device__ __forceinline__ void gemm_tc_pair_persistent(const F &f, float *__res
                     for (int p = 0; p < BH / 32; p += PutB::STEP) {
                         PutB::put(st + OA, tc, p, vb);
 #pragma unroll
-                        for (int i = 0; i < PutB::STEP; i++) fetch_b(S_, it, k0, k_end, p + i);
+                        for (int i = 0; i < PutB::STEP; i++)
+                            if (!ROWS || w < WORK) fetch_b(S_, it, k0, k_end, p + i);
                     }
                 }
             });
