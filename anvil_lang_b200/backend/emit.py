@@ -1059,7 +1059,8 @@ class KernelGen:
         return out
 
     def tc_operands(self, c, touch: bool):
-        """a4 / b4 (four consecutive k of one operand row) and, for fused attention, a_touch / b_touch."""
+        """a4 / b4 (four consecutive k of one operand row) and, with `touch`, a_touch / b_touch (an L2 prefetch; fused attention
+        asks for its next item's operands, the resident template no longer does)."""
         ind = "        "
         dm = self.decode("(uint32_t)m", c.mvars, self.names, ind)
         dn = self.decode("(uint32_t)n", c.nvars, self.names, ind)
@@ -1093,7 +1094,7 @@ class KernelGen:
         M, N, K, NB = c.M, c.N, c.K, c.NB
         nstores = sum(1 for st in k.stmts if isinstance(st, kir.Store))
         variant = tc_variant(c.a_kcontig, M, N, K, nstores)
-        fa4, fb4 = self.tc_operands(c, False)
+        fa4, fb4 = self.tc_operands(c, variant == "pp")
         pp = variant == "pp"
         pair = variant == "pair" or pp
         if pair:                                 # 256 x BN tile per cluster of two CTAs
